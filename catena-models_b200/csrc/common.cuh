@@ -45,15 +45,9 @@ void cm_set_error(const char* fmt, ...);
 //  - the TMA-fed products and the attention kernels trigger when their last loads are under way.
 //    Triggered at once, kernel after kernel became resident and sat waiting, and steps of 1 and
 //    8 sequences took up to 1.5 times as long as without any overlap;
-//  - the weight-streaming product of small decode batches (gemm_skinny.cu) is launched in plain
-//    stream order and triggers as soon as it runs: started early it made those steps 5% slower
-//    (with or without reading weights ahead of its wait, with or without a cluster), while the
-//    TMA-fed products gain from setting up their barriers and tensor memory early (batch 64: 7%
-//    faster).  A chain of spinning kernels of the same shapes gains 40% from starting early, a
-//    chain of these products alone gains nothing (34.9 against 34.1 us for a layer's four): four
-//    blocks of 64 registers fill an SM, so a block that starts early finds room only when one of the
-//    kernel before has left, and what a product spends between launches is mostly the ramp of its
-//    own memory pipeline, which an early start does not shorten.
+//  - the weight-streaming product of small decode batches (gemm_skinny.cu) triggers at once and starts early: its blocks
+//    request their first weights into shared memory and wait with few registers, so that they find room beside the
+//    kernel before (with the weights in registers, four blocks of 64 registers filled an SM and an early start cost 5 %).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -102,17 +102,6 @@ class Runtime:
         the caller can take `kernels.PartialSums` instead (the product cut over K, to be added by the
         fused residual kernel): used where it spares the product an exchange between its blocks."""
         kind = self._product_kernel(x, w)
-        # Partial sums at 9 to 16 rows: the tcgen05 kernel's eight slices beat the streaming kernel's four
-        # (measured on B200 at 16 rows, us: 2,048 x 2,048 5.0 -> 4.0, 2,048 x 8,192 10.4 -> 8.9, 2,048 x 10,752
-        # 13.1 -> 10.1, 1,024 x 4,608 6.1 -> 5.3; at 8 rows the streaming kernel is level or ahead)
-        if (partial_ok and out_dtype is None and kind == "skinny" and 8 < x.shape[0] <= self.SKINNY_BEST_ROWS
-                and w.shape[1] >= 2048 and self._tma_operands(x, w) and self._few_rows_slices(w.shape[0], w.shape[1]) > 1):
-            kind = "few_rows"
-        # ... and so does a finished product of that size (q/k/v at 16 rows: 7.0 -> 6.0 us; in_proj keeps the
-        # streaming kernel, which takes the convolution along)
-        if (not partial_ok and out_dtype is None and kind == "skinny" and 8 < x.shape[0] <= self.SKINNY_BEST_ROWS
-                and w.shape[1] >= 2048 and self._tma_operands(x, w)):
-            kind = "few_rows"
         if partial_ok and out_dtype is None and kind == "skinny" and x.shape[0] <= self.SKINNY_BEST_ROWS:
             slices = self._skinny_slices(w.shape[0], w.shape[1])
             if slices > 1:
@@ -261,6 +250,16 @@ class Runtime:
         that kernel's fused forms, which take no more)."""
         return x.shape[0] <= self.SKINNY_BEST_ROWS and self._product_kernel(x, w) == "skinny"
 
+    def _fills_one_round(self, F):
+        """True where the few-rows product's tiles of 64 gated outputs make one nearly full round over the SMs.  From 9 rows on
+        that kernel then leads the streaming one, whose blocks need more registers for a second set of activation rows (whole
+        decode steps on B200, us, streaming / few-rows: 13 rows over 16,384 x 2,048 weights, 128 tiles for 148 SMs, 1,157 / 1,085;
+        where the tiles make half a round or one and a fraction it does not: 16 rows over 9,216 x 1,024, 72 tiles, 456 / 483;
+        12 rows over 21,504 x 2,048, 168 tiles, 1,498 / 1,577)."""
+        if self._sm_count is None:
+            self._sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
+        return 3 * self._sm_count <= 4 * -(-F // 64) <= 4 * self._sm_count
+
     def gate_up_swiglu(self, x, w_gate_up, F, gelu=False, limit=None):
         """a = act(x Wgate^T) * (x Wup^T) for the row-packed [Wgate; Wup]; act is silu, or with `gelu` the tanh form of
         gelu.  The tensor-core and the streaming products apply it in their epilogues.  `limit` = L: the clamped gate
@@ -269,10 +268,7 @@ class Runtime:
         flag = 3 if limit is not None else (2 if gelu else True)
         limit = float(limit or 0.0)
         kind = self._product_kernel(x, w_gate_up)
-        # From 9 rows on the tcgen05 few-rows kernel leads (measured on B200 at 16 rows, us, streaming /
-        # few-rows: 21,504 x 2,048 weights 25.5 / 20.2, 16,384 x 2,048 15.6 / 14.2, 9,216 x 1,024 7.7 / 7.4; at 8
-        # rows the streaming kernel leads everywhere).
-        if kind == "skinny" and x.shape[0] > 8 and self._tma_operands(x, w_gate_up):
+        if kind == "skinny" and x.shape[0] > 8 and self._tma_operands(x, w_gate_up) and self._fills_one_round(F):
             kind = "few_rows"
         if kind == "skinny":
             kernels.gemm_skinny(a, x, w_gate_up, swiglu=flag, limit=limit)
@@ -292,8 +288,6 @@ class Runtime:
     def linear_gelu(self, x, w):
         """a = gelu(x @ w^T), the tanh form, in x's dtype: in the epilogue of the tensor-core and streaming products."""
         kind = self._product_kernel(x, w)
-        if kind == "skinny" and 8 < x.shape[0] <= self.SKINNY_BEST_ROWS and w.shape[1] >= 2048 and self._tma_operands(x, w):
-            kind = "few_rows"                              # as for a plain product (`linear`)
         a = torch.empty((x.shape[0], w.shape[0]), dtype=x.dtype, device=x.device)
         if kind == "skinny":
             kernels.gemm_skinny(a, x, w, swiglu=kernels.GATE_GELU)
