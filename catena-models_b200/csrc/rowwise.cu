@@ -298,12 +298,207 @@ add_norm_parts_kernel(T* __restrict__ h_out, T* __restrict__ n_out,
     }
 }
 
+// The same for many bfloat16 rows of at most 2,048 elements: a warp per row instead of a block.  The form above spends
+// two barriers a sum and a block's launch on each row and fetches 16 KB of weights per row; it reached 2.6 to 3.3 TB/s
+// (16,384 x 2,048 82 us, 70,442 x 1,024 221 us, where half of each block's threads hold nothing).  Here one block an SM
+// walks rows, the weights wait in shared memory, and every warp has its next rows on their way (cp.async) while it works on
+// one: 59 and 95 us (4.5 and 6.1 TB/s; with loads into registers at the row's start 71 and 138).  The sums are
+// formed in the order of the form above, in which lane l of warp j held elements 256 j + 8 l ..: this lane's eighth j
+// holds those, eight sums are reduced over the lanes together (each step adds the same pairs as a butterfly of one sum
+// would, and halves what a lane still carries), and then over j as the block's second step does: the bits are the same.
+#define NVR_MAX_WIDTH 2048
+
+__device__ __forceinline__ float nvr_row_sum(float (&v)[8], int lane) {
+#pragma unroll
+    for (int half = 4, o = 16; half >= 1; half >>= 1, o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int j = 0; j < half; ++j) {
+            const float mine = upper ? v[j + half] : v[j], theirs = upper ? v[j] : v[j + half];
+            v[j] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+        }
+    }
+    // the lane's eighth j is given by its bits 4, 3, 2; the sum over its lanes still wants bits 1 and 0
+    float t = v[0];
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 16);              // over j: bits 2, 1, 0 of j in this order
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+    t += __shfl_xor_sync(0xffffffffu, t, 4);
+    return t;
+}
+
+__device__ __forceinline__ void nvr_unpack(const uint4& raw, float* out) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]);
+        out[2 * i] = f.x;
+        out[2 * i + 1] = f.y;
+    }
+}
+
+// J: eighths of 256 elements that a row needs, H <= 256 J; WARPS rows at a time, BUFS buffers of a row each (m beside h)
+template <int J, int WARPS, int BUFS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+add_norm_rows_kernel(bf16* __restrict__ h_out, bf16* __restrict__ n_out, const bf16* __restrict__ m,
+                     const bf16* __restrict__ h_in, const float* __restrict__ w_post, const float* __restrict__ w_next,
+                     int rows, int H, float eps_post, float eps_next) {
+    extern __shared__ __align__(16) float4 nvr_smem[];
+    // the two halves of each run of eight weights apart: no bank conflicts
+    float4 (*wp_s)[J * 32] = reinterpret_cast<float4 (*)[J * 32]>(nvr_smem);
+    float4 (*wn_s)[J * 32] = reinterpret_cast<float4 (*)[J * 32]>(nvr_smem + 2 * J * 32);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4* buf = reinterpret_cast<uint4*>(nvr_smem + 4 * J * 32) + warp * (BUFS * 2 * J * 32);
+    const uint32_t buf_addr = (uint32_t)__cvta_generic_to_shared(buf);
+    pdl_trigger();
+    for (int c = threadIdx.x; c < J * 32; c += WARPS * 32) {
+        if (c * 8 >= H) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (w_post) wp_s[h][c] = *reinterpret_cast<const float4*>(w_post + c * 8 + h * 4);
+            if (w_next) wn_s[h][c] = *reinterpret_cast<const float4*>(w_next + c * 8 + h * 4);
+        }
+    }
+    __syncthreads();
+    pdl_wait();
+    const int step = gridDim.x * WARPS;
+    auto fetch = [&](int row, int slot) {
+        if (row < rows) {
+            const long long off = (long long)row * H;
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const int e = (j * 32 + lane) * 8;
+                if (e < H) {
+                    const uint32_t dst = buf_addr + ((slot * 2 * J + j) * 32 + lane) * 16;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(m + off + e) : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + J * 512), "l"(h_in + off + e) : "memory");
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int first = blockIdx.x * WARPS + warp;
+#pragma unroll
+    for (int i = 0; i < BUFS - 1; ++i) fetch(first + i * step, i);
+    int slot = 0;
+    for (int row = first; row < rows; row += step) {
+        fetch(row + (BUFS - 1) * step, slot == 0 ? BUFS - 1 : slot - 1);       // the buffer of the row before
+        asm volatile("cp.async.wait_group %0;" ::"n"(BUFS - 1) : "memory");    // a lane reads only what it copied itself
+        const long long off = (long long)row * H;
+        uint4 mr[J], hr[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int e = (j * 32 + lane) * 8;
+            mr[j] = hr[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (e < H) {
+                mr[j] = buf[(slot * 2 * J + j) * 32 + lane];
+                hr[j] = buf[(slot * 2 * J + J + j) * 32 + lane];
+            }
+        }
+        slot = slot + 1 == BUFS ? 0 : slot + 1;
+        float s[8];
+        float inv_post = 1.f;
+        if (w_post) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                s[j] = 0.f;
+                if (j < J) {
+                    float v[8];
+                    nvr_unpack(mr[j < J ? j : 0], v);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) s[j] += v[i] * v[i];
+                }
+            }
+            inv_post = 1.f / sqrtf(nvr_row_sum(s, lane) / (float)H + eps_post);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            s[j] = 0.f;
+            if (j < J) {
+                const int e = (j * 32 + lane) * 8;
+                float mv[8], hv[8], wv[8];
+                nvr_unpack(mr[j < J ? j : 0], mv);
+                nvr_unpack(hr[j < J ? j : 0], hv);
+                if (w_post && e < H) {
+                    *reinterpret_cast<float4*>(wv) = wp_s[0][j * 32 + lane];
+                    *reinterpret_cast<float4*>(wv + 4) = wp_s[1][j * 32 + lane];
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float d = w_post ? rounded<bf16>((mv[i] * inv_post) * wv[i]) : mv[i];
+                    hv[i] = rounded<bf16>(hv[i] + d);
+                    if (e < H) s[j] += hv[i] * hv[i];
+                }
+                __nv_bfloat162* packed = reinterpret_cast<__nv_bfloat162*>(&hr[j < J ? j : 0]);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) packed[i] = __floats2bfloat162_rn(hv[2 * i], hv[2 * i + 1]);
+                if (e < H) *reinterpret_cast<uint4*>(h_out + off + e) = hr[j < J ? j : 0];
+            }
+        }
+        if (!w_next) continue;
+        const float inv_next = 1.f / sqrtf(nvr_row_sum(s, lane) / (float)H + eps_next);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int e = (j * 32 + lane) * 8;
+            if (e >= H) continue;
+            float hv[8], wv[8], o[8];
+            nvr_unpack(hr[j], hv);
+            *reinterpret_cast<float4*>(wv) = wn_s[0][j * 32 + lane];
+            *reinterpret_cast<float4*>(wv + 4) = wn_s[1][j * 32 + lane];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = (hv[i] * inv_next) * wv[i];
+            store8f<bf16>(n_out + off + e, o);
+        }
+    }
+}
+
 #define NV_BLOCKS_PER_SM 4
+// From here on a warp per row (four times as many from 1,025 elements on, where an SM's block holds 12 rows at a time: 2,048
+// x 2,048 are 1.15 rounds of rows over the warps, 15.8 us against 13.7).
+#define NVR_MIN_ROWS 1024
+
+static int nv_sm_count() {
+    static int sm_count = 0;
+    if (!sm_count) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+        if (sm_count <= 0) sm_count = 1;
+    }
+    return sm_count;
+}
+
+template <int J, int WARPS, int BUFS>
+static int launch_add_norm_rows(bf16* h_out, bf16* n_out, const bf16* m, const bf16* h_in, const float* w_post, const float* w_next,
+                                int rows, int H, float eps_post, float eps_next, cudaStream_t st) {
+    constexpr size_t smem = (4 + WARPS * BUFS * 2) * J * 32 * 16;
+    auto kernel = add_norm_rows_kernel<J, WARPS, BUFS>;
+    static bool configured = false;
+    if (!configured) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+            cudaGetLastError();
+            cm_set_error("add_norm: %zu bytes of shared memory refused", smem);
+            return CM_ERR_LAUNCH;
+        }
+        configured = true;
+    }
+    const int want = (rows + WARPS - 1) / WARPS, sms = nv_sm_count();
+    cm_launch(kernel, want < sms ? want : sms, WARPS * 32, smem, st, h_out, n_out, m, h_in, w_post, w_next, rows, H, eps_post, eps_next);
+    CM_CHECK_LAUNCH();
+    return CM_OK;
+}
 
 template <typename T>
 static int launch_add_norm(void* h_out, void* n_out, const void* m, const void* h_in, const float* w_post,
                            const float* w_next, int rows, int H, float eps_post, float eps_next, cudaStream_t st) {
     const int chunks = (H / 8 + NV_THREADS - 1) / NV_THREADS;
+    if (sizeof(T) == 2 && H <= NVR_MAX_WIDTH && rows >= (H <= 1024 ? NVR_MIN_ROWS : 4 * NVR_MIN_ROWS)) {
+        const bf16 *mm = (const bf16*)m, *hh = (const bf16*)h_in;
+        if (H <= 512) return launch_add_norm_rows<2, 16, 4>((bf16*)h_out, (bf16*)n_out, mm, hh, w_post, w_next, rows, H, eps_post, eps_next, st);
+        if (H <= 1024) return launch_add_norm_rows<4, 16, 3>((bf16*)h_out, (bf16*)n_out, mm, hh, w_post, w_next, rows, H, eps_post, eps_next, st);
+        return launch_add_norm_rows<8, 12, 2>((bf16*)h_out, (bf16*)n_out, mm, hh, w_post, w_next, rows, H, eps_post, eps_next, st);
+    }
     if (chunks <= 1)
         cm_launch(add_norm_kernel<T, 1>, rows, NV_THREADS, 0, st, (T*)h_out, (T*)n_out, (const T*)m, (const T*)h_in, w_post,
                   w_next, H, eps_post, eps_next);
@@ -322,13 +517,7 @@ static int launch_add_norm_parts(void* h_out, void* n_out, const float* m_parts,
                                  const void* h_in, const float* w_post, const float* w_next, int rows, int H,
                                  float eps_post, float eps_next, cudaStream_t st) {
     const int chunks = (H / 8 + NV_THREADS - 1) / NV_THREADS;
-    static int sm_count = 0;
-    if (!sm_count) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        if (sm_count <= 0) sm_count = 1;
-    }
+    const int sm_count = nv_sm_count();
     const int blocks = rows < NV_BLOCKS_PER_SM * sm_count ? rows : NV_BLOCKS_PER_SM * sm_count;
     if (chunks <= 1)
         cm_launch(add_norm_parts_kernel<T, 1>, blocks, NV_THREADS, 0, st, (T*)h_out, (T*)n_out, m_parts, n_parts,

@@ -171,6 +171,143 @@ shortconv_vec_kernel(T* __restrict__ y, const T* __restrict__ bcx, long long ld,
     }
 }
 
+// Many tokens: a thread owns eight channels of eight (bfloat16) or four consecutive tokens.  The form above forms each token's B * X product
+// again for every tap that reads it (seven 16-byte loads a token with three taps, four of them from L1: 16,384 x 2,048
+// took 95 us, 70,442 x 1,024 about 300); here a product is formed once and stays in registers for the K - 1 tokens after
+// it, and all loads of the run are in flight together: 83 and 146 us (with each token's sequence looked up when its turn
+// came 97 and 166).  The same multiplications and additions in the same order.
+#define SCR_ROWS(T) (sizeof(T) == 2 ? 8 : 4)
+#define SCR_MIN_TOKENS 1024
+
+template <typename T>
+struct Raw8 { uint4 v[sizeof(T) / 2]; };               // eight elements as they lie in memory
+template <typename T>
+__device__ __forceinline__ Raw8<T> raw8(const T* p) {
+    Raw8<T> r;
+#pragma unroll
+    for (int i = 0; i < (int)sizeof(T) / 2; ++i) r.v[i] = reinterpret_cast<const uint4*>(p)[i];
+    return r;
+}
+__device__ __forceinline__ void unpack8(const Raw8<bf16>& r, float* out) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __bfloat1622float2(h[i]);
+        out[2 * i] = f.x;
+        out[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void unpack8(const Raw8<float>& r, float* out) {
+    const float* f = reinterpret_cast<const float*>(&r);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[i] = f[i];
+}
+
+template <typename T, int K>
+__global__ void __launch_bounds__(128)
+shortconv_rows_kernel(T* __restrict__ y, const T* __restrict__ bcx, long long ld, const float* __restrict__ w_t,
+                      float* __restrict__ state, const int* __restrict__ tok_seq, const int* __restrict__ seq_start,
+                      const int* __restrict__ seq_slot, const int* __restrict__ seq_pos0, int T_tokens, int H, int from_zero,
+                      int phase) {
+    constexpr int ROWS = SCR_ROWS(T);
+    pdl_trigger();
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+    const int t0 = (blockIdx.x * blockDim.y + threadIdx.y) * ROWS;
+    float w[K][8];
+    if (c < H)
+#pragma unroll
+        for (int j = 0; j < K; ++j) load8f<float>(w_t + (long long)j * H + c, w[j]);
+    pdl_wait();
+    if (c >= H || t0 >= T_tokens) return;
+    // which sequence each token belongs to, and where in it the token stands: asked for with the rows, not token by token
+    int seq[ROWS], at[ROWS], left[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) seq[q] = tok_seq[min(t0 + q, T_tokens - 1)];
+    Raw8<T> rb[ROWS + K - 1], rx[ROWS + K - 1], rc[ROWS];      // B and X of the tokens t0 - K + 1 .. (those outside: repeated, unused)
+#pragma unroll
+    for (int q = 0; q < ROWS + K - 1; ++q) {
+        const int t = min(max(t0 + q - (K - 1), 0), T_tokens - 1);
+        rb[q] = raw8<T>(bcx + (long long)t * ld + c);
+        rx[q] = raw8<T>(bcx + (long long)t * ld + 2 * H + c);
+        if (q >= K - 1) rc[q - (K - 1) < 0 ? 0 : q - (K - 1)] = raw8<T>(bcx + (long long)t * ld + H + c);
+    }
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        at[q] = t0 + q - seq_start[max(seq[q], 0)];
+        left[q] = seq_start[max(seq[q], 0) + 1] - (t0 + q);            // 1 at a sequence's last token
+    }
+    float bx[K][8];                                    // of the tokens t - K + 1 .. t, whatever sequence they belong to
+    auto product = [&](int q, float (&v)[8]) {
+        float bb[8], xx[8];
+        unpack8(rb[q], bb);
+        unpack8(rx[q], xx);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = bb[e] * xx[e];
+    };
+#pragma unroll
+    for (int j = 1; j < K; ++j) product(j - 1, bx[j]);
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int t = t0 + q;
+        if (t >= T_tokens) return;
+#pragma unroll
+        for (int j = 0; j + 1 < K; ++j)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) bx[j][e] = bx[j + 1][e];
+        product(q + K - 1, bx[K - 1]);
+        float cc[8], out[8];
+        unpack8(rc[q], cc);
+        if (seq[q] < 0) {                             // a row of padding belongs to no sequence: zeros out
+#pragma unroll
+            for (int e = 0; e < 8; ++e) out[e] = 0.f;
+            store8f<T>(y + (long long)t * H + c, out);
+            continue;
+        }
+        const int i = at[q];
+        // the stored state of the token's sequence, or null for one that starts from nothing (looked up at its ends only)
+        const float* before = nullptr;
+        if (i < K - 1 && !from_zero && !(seq_pos0 && seq_pos0[seq[q]] == 0)) before = state + (long long)seq_slot[seq[q]] * (K - 1) * H + c;
+        float z[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) z[e] = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            const int r = i + j - (K - 1);
+            if (r < 0) {                              // one of the sequence's first tokens: from the state
+                float sv[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) sv[e] = 0.f;
+                if (before) load8f<float>(before + (long long)(K - 1 + r) * H, sv);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) z[e] += w[j][e] * sv[e];
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) z[e] += w[j][e] * bx[j][e];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) out[e] = z[e] * cc[e];
+        store8f<T>(y + (long long)t * H + c, out);
+        if (left[q] == 1 && phase != 1) {
+            const int len = i + 1;
+            float* st = state + (long long)seq_slot[seq[q]] * (K - 1) * H + c;
+#pragma unroll
+            for (int j = 0; j + 1 < K; ++j) {         // new entry j = s[len + j]; s below K - 1 is an old entry
+                const int r = len + j - (K - 1);
+                if (r >= 0) {
+                    store8f<float>(st + (long long)j * H, bx[j + 1]);
+                } else {
+                    float sv[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) sv[e] = 0.f;
+                    if (before) load8f<float>(before + (long long)(len + j) * H, sv);       // len + j > j: not yet overwritten
+                    store8f<float>(st + (long long)j * H, sv);
+                }
+            }
+        }
+    }
+}
+
 // w: taps [H][K]; w_t: the same taps stored [K][H] (optional; lets the vector kernel read them
 // eight channels at a time).
 extern "C" int cm_shortconv(int dt, void* y, const void* bcx, long long ld, const float* w, const float* w_t,
@@ -184,6 +321,26 @@ extern "C" int cm_shortconv(int dt, void* y, const void* bcx, long long ld, cons
     const int last_phase = first_phase ? 2 : 0;
     for (int phase = first_phase; phase <= last_phase; ++phase) {
     const bool vec = H % 8 == 0 && ld % 8 == 0 && (((uintptr_t)y | (uintptr_t)bcx | (uintptr_t)state) & 15) == 0;
+    if (vec && w_t && K <= 4 && T >= SCR_MIN_TOKENS && phase != 2 && !one_token_each && ((uintptr_t)w_t & 15) == 0) {
+        const int run = 4 * (dt == DT_F32 ? SCR_ROWS(float) : SCR_ROWS(bf16));
+        const dim3 rblock(32, 4), rgrid((T + run - 1) / run, (H / 8 + 31) / 32);
+#define SC_LAUNCH_ROWS(TT, KT)                                                                                        \
+    cm_launch(shortconv_rows_kernel<TT, KT>, rgrid, rblock, 0, st, (TT*)y, (const TT*)bcx, ld, w_t, state, tok_seq, seq_start, \
+              seq_slot, seq_pos0, T, H, from_zero, phase)
+        if (dt == DT_F32) {
+            if (K == 2) SC_LAUNCH_ROWS(float, 2);
+            else if (K == 3) SC_LAUNCH_ROWS(float, 3);
+            else SC_LAUNCH_ROWS(float, 4);
+        } else if (dt == DT_BF16) {
+            if (K == 2) SC_LAUNCH_ROWS(bf16, 2);
+            else if (K == 3) SC_LAUNCH_ROWS(bf16, 3);
+            else SC_LAUNCH_ROWS(bf16, 4);
+        } else {
+            return CM_ERR_DTYPE;
+        }
+        CM_CHECK_LAUNCH();
+        continue;
+    }
     if (vec) {
         // few tokens: a token per block (128 channel groups); many: 4 consecutive tokens per block
         const int ty = T >= 256 ? 4 : 1, tx = 128 / ty;
