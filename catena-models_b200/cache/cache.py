@@ -228,21 +228,15 @@ class Cache:
         if book.length[dst] != 0 or any(book.pages[dst]):
             raise CacheError(f"copy_slot: slot {dst} already holds tokens")
         length = book.length[src]
-        updates = book.reserve(dst, length)                  # raises CacheFull and takes nothing if short
-        flat = self.flat_updates(dst, updates)
-        if flat:
-            index = torch.tensor([i for i, _ in flat], dtype=torch.int32, device=self.device)
-            value = torch.tensor([p for _, p in flat], dtype=torch.int32, device=self.device)
-            count = torch.tensor([len(flat)], dtype=torch.int32, device=self.device)
-            kernels.scatter_i32(self.ptab_all, index, value, count, len(flat))
+        book.reserve(dst, length)                            # raises CacheFull and takes nothing if short
         for g in range(len(self.kv_specs)):
-            n = len(book.pages[dst][g])
-            if n:
-                s_ids = torch.tensor(book.pages[src][g][:n], dtype=torch.int32, device=self.device)
-                d_ids = torch.tensor(book.pages[dst][g], dtype=torch.int32, device=self.device)
-                kernels.copy_pages(self.kv_storage[g], s_ids, d_ids)
+            pages = book.pages[dst][g]                       # all of them new: the slot's page table from its start
+            kernels.copy_pages_ids(self.kv_storage[g], book.pages[src][g][:len(pages)], pages, 2, self.ptabs[g][dst, :len(pages)])
         for store in self.fixed_storage:
-            store[:, dst].copy_(store[:, src])
+            if store[0, 0].numel() * store.element_size() % 16 == 0:
+                kernels.copy_pages_ids(store, [src], [dst], 1)
+            else:
+                store[:, dst].copy_(store[:, src])
         book.advance(dst, length)
 
     def flat_updates(self, slot, updates):

@@ -101,6 +101,55 @@ __global__ void copy_pages_kernel(uint4* __restrict__ pool, const int* __restric
     for (long long i = threadIdx.x; i < page_vec; i += blockDim.x) to[i] = from[i];
 }
 
+// The same with the page ids in the launch's arguments instead of device memory, a few hundred at a time, and (ptab given)
+// the copy's page-table entries ptab[0 .. n-1] = dst written on the way: a resumed sequence's whole state then takes a
+// launch per group and no host-to-device copy.  (With six id tensors a sequence, each of whose copies waits for the stream,
+// resuming 64 sequences took 9 ms of a 74 ms pass; the pages' own bytes take about 12 us a sequence.)
+#define CP_MAX 256
+struct CopyIds {
+    int src[CP_MAX], dst[CP_MAX];
+};
+__global__ void copy_pages_ids_kernel(uint4* __restrict__ pool, CopyIds ids, long long pages, long long page_vec, int* __restrict__ ptab) {
+    pdl_trigger();
+    pdl_wait();
+    const int dst = ids.dst[blockIdx.x];
+    if (ptab && blockIdx.y == 0 && threadIdx.x == 0) ptab[blockIdx.x] = dst;
+    const long long plane = (long long)blockIdx.y * pages;
+    const uint4* from = pool + (plane + ids.src[blockIdx.x]) * page_vec;
+    uint4* to = pool + (plane + dst) * page_vec;
+    long long i = threadIdx.x;
+    for (; i + 3LL * blockDim.x < page_vec; i += 4LL * blockDim.x) {           // four loads in flight per thread
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = __ldcs(from + i + (long long)u * blockDim.x);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) to[i + (long long)u * blockDim.x] = v[u];
+    }
+    for (; i < page_vec; i += blockDim.x) to[i] = from[i];
+}
+
+extern "C" int cm_copy_pages_ids(void* pool, const int* src, const int* dst, int n, int outer, long long pages, long long page_bytes,
+                                 int* ptab, cudaStream_t st) {
+    if (n <= 0 || outer <= 0) return CM_OK;
+    if (page_bytes % 16 || (reinterpret_cast<uintptr_t>(pool) & 15))
+        CM_REFUSE("copy_pages: pages of %lld bytes (multiples of 16, 16-byte aligned pool)", page_bytes);
+    if (outer > 65535) CM_REFUSE("copy_pages: %d planes", outer);
+    for (int i = 0; i < n; ++i)
+        if (src[i] < 0 || src[i] >= pages || dst[i] < 0 || dst[i] >= pages) CM_REFUSE("copy_pages: page %d to %d of %lld", src[i], dst[i], pages);
+    for (int first = 0; first < n; first += CP_MAX) {
+        CopyIds ids;
+        const int count = n - first < CP_MAX ? n - first : CP_MAX;
+        for (int i = 0; i < count; ++i) {
+            ids.src[i] = src[first + i];
+            ids.dst[i] = dst[first + i];
+        }
+        cm_launch(copy_pages_ids_kernel, dim3(count, outer), 256, 0, st, (uint4*)pool, ids, pages, page_bytes / 16,
+                  ptab ? ptab + first : nullptr);
+        CM_CHECK_LAUNCH();
+    }
+    return CM_OK;
+}
+
 extern "C" int cm_copy_pages(void* pool, const int* src, const int* dst, int n, int outer, long long pages,
                              long long page_bytes, cudaStream_t st) {
     if (n <= 0 || outer <= 0) return CM_OK;

@@ -7,6 +7,7 @@ cannot be built or loaded, importing a kernel raises.
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 
 import torch
@@ -52,6 +53,7 @@ _SIGNATURES = {
     "cm_sample": [_vp, _vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp],
     "cm_scatter_i32": [_vp, _vp, _vp, _vp, _i, _vp],
     "cm_zero_slots": [_vp, _i, _ll, _ll, ctypes.POINTER(ctypes.c_int), _i, _vp],
+    "cm_copy_pages_ids": [_vp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), _i, _i, _ll, _ll, _vp, _vp],
     "cm_copy_pages": [_vp, _vp, _vp, _i, _i, _ll, _ll, _vp],
     "cm_norm_f32in": [_i, _vp, _vp, _vp, _i, _i, _f, _i, _vp, _vp, _vp],
     "cm_residual_add_norm": [_i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp, _vp, _vp],
@@ -815,6 +817,20 @@ def copy_pages(pool, src, dst):
     outer, pages = pool.shape[0] * pool.shape[1], pool.shape[2]
     page_bytes = pool[0, 0, 0].numel() * pool.element_size()
     _check(lib().cm_copy_pages(_ptr(pool), _ptr(src), _ptr(dst), n, outer, pages, page_bytes, _stream()), "copy_pages")
+
+
+def copy_pages_ids(pool, src, dst, outer_dims, ptab=None):
+    """`copy_pages` with the page numbers as Python ints: pool [outer dimensions (`outer_dims` of them), pages, ...]; with
+    `ptab` (int32, one entry per page copied) the new pages are written there too."""
+    if not src:
+        return
+    if len(src) != len(dst) or (ptab is not None and (ptab.numel() != len(dst) or ptab.dtype != torch.int32 or not ptab.is_contiguous())):
+        raise KernelError("copy_pages_ids: one new page, and one page-table entry, per page copied")
+    outer, pages = math.prod(pool.shape[:outer_dims]), pool.shape[outer_dims]
+    page_bytes = math.prod(pool.shape[outer_dims + 1:]) * pool.element_size()
+    ids = ctypes.c_int * len(src)
+    _check(lib().cm_copy_pages_ids(_ptr(pool), ids(*src), ids(*dst), len(src), outer, pages, page_bytes,
+                                   _ptr(ptab), _stream()), "copy_pages", -(-len(src) // 256))
 
 
 def zero_slots(store, slots):
