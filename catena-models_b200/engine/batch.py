@@ -16,8 +16,21 @@ touch no cache and change no result; recorded prompt steps use them to serve a c
 """
 from __future__ import annotations
 
+import array
+
 import numpy as np
 import torch
+
+
+def token_array(tokens):
+    """A sequence's token ids as an integer array, converted once for the checks and for the step's buffer.  A list of ints
+    goes through `array`, which takes a third of numpy's time for it; whatever that refuses is left to numpy."""
+    if type(tokens) is list:
+        try:
+            return np.frombuffer(array.array("q", tokens), dtype=np.int64)
+        except (TypeError, OverflowError):
+            pass
+    return np.asarray(tokens)
 
 
 class BatchLayout:

@@ -30,7 +30,7 @@ from ..cache.cache import Cache
 from ..cache.allocators import CacheError, CacheFull
 from .. import kernels as _kernels
 from ..csrc.limits import PAGE_TOKENS
-from .batch import BatchLayout, StepBatch, clear_sampling, fill_host, fill_host_decode, fill_sampling
+from .batch import BatchLayout, StepBatch, clear_sampling, fill_host, fill_host_decode, fill_sampling, token_array
 
 
 PROMPT_GRAPH_MAX_TOKENS = 1024     # longer prompt steps are bound by the device, not by their launches
@@ -186,8 +186,8 @@ class Engine:
                 raise StepError("this model has a part without an append form: its sequences either all "
                                 "start at their first token or all go on by one token")
         V = self.model.vocab_size
-        for t in tokens:
-            arr = np.asarray(t)
+        arrays = [token_array(t) for t in tokens]
+        for arr in arrays:
             if arr.min() < 0 or arr.max() >= V:
                 raise StepError(f"token id outside the vocabulary of {V}")
         if want is None:
@@ -197,7 +197,7 @@ class Engine:
         for w, t in zip(want, tokens):
             if any(i < 0 or i >= len(t) for i in w):
                 raise StepError("a wanted place lies outside the sequence's tokens of this step")
-        return positions, kind, want
+        return positions, kind, want, arrays
 
     def _reserve(self, slots, positions, tokens):
         """Pages for the new tokens of every sequence; undone as a whole if one does not fit."""
@@ -268,7 +268,7 @@ class Engine:
             for s, p in zip(slots, positions):
                 book.length[s] = p + 1
         else:
-            positions, kind, want = self._check(slots, tokens, want)
+            positions, kind, want, arrays = self._check(slots, tokens, want)
             updates = self._reserve(slots, positions, tokens)
             B, T = len(slots), sum(len(t) for t in tokens)
             if kind == "decode" and self.use_graphs:
@@ -278,7 +278,7 @@ class Engine:
                     logits = logits[[b for b, w in enumerate(want) for _ in w]]
             else:
                 self._sampled_count = 0                        # what this step samples does not land in `_sampled`
-                logits, sampled = self._prompt_step(slots, tokens, positions, kind, want, updates, sampling)
+                logits, sampled = self._prompt_step(slots, arrays, positions, kind, want, updates, sampling)
             for s, p, t in zip(slots, positions, tokens):
                 book.advance(s, p + len(t))
         self.steps_run += 1
