@@ -207,11 +207,12 @@ gemm_simt_rows_kernel(float* __restrict__ Y, const float* __restrict__ X, const 
 
 // ---- float, 16-byte aligned operands, many rows -----------------------------------------------------------
 // BM x 128 outputs a block, 2 BM threads of 8 x 8 each: rows ty * 4 (+ BM / 2), columns tx * 4 (+ 64).  Operands are
-// kept k-major in shared memory (two buffers of 16 k, filled from registers while the other is multiplied); columns are
+// kept k-major in shared memory (two buffers of 16 k); columns are
 // multiplied in packed pairs (fma.rn.f32x2: each half is an IEEE fused multiply-add, as the scalar one; with scalar ones
 // 1,000 x 9,216 x 1,024 took 515 us in place of 410).  The sums over whole slices are kept in shared memory, which leaves
-// registers for two blocks of 128 rows per SM (with them in registers, one block: 473 us).  Bound by the FMA pipe: 46 of the
-// 75 TFLOP/s at 1,000 x 9,216 x 1,024.
+// registers for two blocks per SM (128 rows with them in registers, one block: 473 us).  Bound by the FMA pipe where tiles fill
+// the device: 46 of the 75 TFLOP/s at 1,000 x 9,216 x 1,024.  With one block of 64 rows an SM it was the loads, a k-step (0.5 us
+// of arithmetic) ahead: a ring of four k-steps took 1,000 x 1,024 x 4,608 from 455 to 286 us.
 #define GST_BN 128
 #define GST_BK 16
 
@@ -224,16 +225,22 @@ __device__ __forceinline__ void gs_fma2(uint64_t& d, uint64_t a, uint64_t b) { a
 __device__ __forceinline__ void gs_add2(uint64_t& d, uint64_t a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
 
 template <int BM>
-__global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 3)
+__global__ void __launch_bounds__(2 * BM, 2)
 gemm_simt_tile_kernel(float* __restrict__ Y, const float* __restrict__ X, const float* __restrict__ W, int M, int N, int K,
                       long long ldx, long long ldw, long long ldy) {
     constexpr int THREADS = 2 * BM;
     constexpr int LW = 512 / THREADS;                                  // 16-byte pieces of W per thread and k-step (of X: 2)
     constexpr int ROWS = THREADS / 4;                                  // rows that one piece of every thread covers
+    // RAW > 0: the operands come through a ring of RAW k-steps in shared memory, as they lie in memory (cp.async), and a thread
+    // moves the pieces that it copied itself into the k-major buffers when their step is next: a lone block's loads then have
+    // RAW k-steps to arrive instead of one.  RAW 0: through registers, one step ahead (two blocks an SM cover for each other).
+    constexpr int RAW = BM == 64 ? 4 : 0;
+    constexpr int PIECES = 2 + LW;                                     // 16-byte pieces of a k-step per thread
     extern __shared__ __align__(16) float gst_smem[];
     uint64_t* total = reinterpret_cast<uint64_t*>(gst_smem);           // [32][THREADS]: a thread's sums over whole slices
     float (*xs)[GST_BK][BM + 4] = reinterpret_cast<float (*)[GST_BK][BM + 4]>(gst_smem + 64 * THREADS);
     float (*ws)[GST_BK][GST_BN + 4] = reinterpret_cast<float (*)[GST_BK][GST_BN + 4]>(gst_smem + 64 * THREADS + 2 * GST_BK * (BM + 4));
+    float4* raw = reinterpret_cast<float4*>(gst_smem + 64 * THREADS + 2 * GST_BK * (BM + 4 + GST_BN + 4));      // [RAW][PIECES][THREADS]
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * GST_BN;
     const int lr = tid >> 2, lk = (tid & 3) * 4;
@@ -244,6 +251,30 @@ gemm_simt_tile_kernel(float* __restrict__ Y, const float* __restrict__ X, const 
         for (int j = 0; j < 4; ++j) acc[i][j] = 0;
     float4 xa[2], wa[LW];
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto copy_w = [&](int step) {
+#pragma unroll
+        for (int i = 0; i < LW; ++i) {
+            const int r = n0 + lr + ROWS * i, k = step * GST_BK + lk;
+            const bool ok = r < N && k < K;
+            gs_cp16((uint32_t)__cvta_generic_to_shared(raw + ((step % (RAW ? RAW : 1)) * PIECES + 2 + i) * THREADS + tid),
+                    ok ? W + (long long)r * ldw + k : W, ok);
+        }
+    };
+    auto copy_x = [&](int step) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int r = m0 + lr + ROWS * i, k = step * GST_BK + lk;
+            const bool ok = r < M && k < K;
+            gs_cp16((uint32_t)__cvta_generic_to_shared(raw + ((step % (RAW ? RAW : 1)) * PIECES + i) * THREADS + tid),
+                    ok ? X + (long long)r * ldx + k : X, ok);
+        }
+    };
+    auto take = [&](int step) {                                        // this thread's pieces of a step that has arrived
+#pragma unroll
+        for (int i = 0; i < 2; ++i) xa[i] = raw[((step % (RAW ? RAW : 1)) * PIECES + i) * THREADS + tid];
+#pragma unroll
+        for (int i = 0; i < LW; ++i) wa[i] = raw[((step % (RAW ? RAW : 1)) * PIECES + 2 + i) * THREADS + tid];
+    };
     auto fetch_w = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < LW; ++i) {
@@ -272,15 +303,37 @@ gemm_simt_tile_kernel(float* __restrict__ Y, const float* __restrict__ X, const 
             for (int j = 0; j < 4; ++j) ws[b][lk + j][lr + ROWS * i] = v[j];
         }
     };
-    fetch_w(0);
-    pdl_wait();
-    fetch_x(0);
+    const int steps = (K + GST_BK - 1) / GST_BK;
+    if (RAW) {
+#pragma unroll
+        for (int i = 0; i < RAW; ++i)
+            if (i < steps) copy_w(i);
+        pdl_wait();
+#pragma unroll
+        for (int i = 0; i < RAW; ++i) {
+            if (i < steps) copy_x(i);
+            asm volatile("cp.async.commit_group;" ::: "memory");       // the first group holds every weight requested above
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(RAW > 0 ? RAW - 1 : 0) : "memory");
+        take(0);
+    } else {
+        fetch_w(0);
+        pdl_wait();
+        fetch_x(0);
+    }
     put(0);
     __syncthreads();
     int b = 0;
     for (int k0 = 0; k0 < K; k0 += GST_BK, b ^= 1) {
         const bool more = k0 + GST_BK < K;
-        if (more) {
+        if (RAW) {
+            const int next = k0 / GST_BK + RAW;                        // into the place of the step in the buffers now
+            if (next < steps) {
+                copy_w(next);
+                copy_x(next);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        } else if (more) {
             fetch_w(k0 + GST_BK);
             fetch_x(k0 + GST_BK);
         }
@@ -318,7 +371,13 @@ gemm_simt_tile_kernel(float* __restrict__ Y, const float* __restrict__ X, const 
                     }
                 }
         }
-        if (more) put(b ^ 1);
+        if (more) {
+            if (RAW) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(RAW > 0 ? RAW - 1 : 0) : "memory");
+                take(k0 / GST_BK + 1);
+            }
+            put(b ^ 1);
+        }
         __syncthreads();
     }
     pdl_trigger();
@@ -375,7 +434,7 @@ static int launch_simt_rows(float* Y, const float* X, const float* W, int M, int
 template <int BM>
 static int launch_simt_tile(float* Y, const float* X, const float* W, int M, int N, int K, long long ldx, long long ldw,
                             long long ldy, cudaStream_t st) {
-    constexpr size_t smem = (64 * 2 * BM + 2 * GST_BK * (BM + 4 + GST_BN + 4)) * 4;
+    constexpr size_t smem = (64 * 2 * BM + 2 * GST_BK * (BM + 4 + GST_BN + 4) + (BM == 64 ? 4 * GST_BK * (BM + GST_BN) : 0)) * 4;
     auto kernel = gemm_simt_tile_kernel<BM>;
     static bool configured = false;
     if (!configured) {
@@ -396,9 +455,10 @@ static int launch_simt_tile(float* Y, const float* X, const float* W, int M, int
 //    with 16 rows a warp 9.3, before 527), else 16 (4 x 9,216 x 1,024: 13.1 / 11.4, before 119);
 //  - up to 8 rows: one pass of eight (8 x 9,216 x 1,024 14.0), or two of four for a narrow W (8 x 1,024 x 1,024 3.3 / 3.9);
 //  - more: whichever of the passes of eight rows and the two tiles is estimated faster.  A pass costs its arithmetic at
-//    15.5 TFLOP/s (128 x 1,024 x 4,608: 87 us, before 510); a tile costs 0.087 us (64 rows) or 0.123 us (128) per k where it has an SM
-//    to itself and 0.056 or 0.100 us where tiles share one: 250 x 9,216 x 1,024 127 and 162 us (passes 305, before
-//    300), 1,000 x 16,384 x 2,048 1,530 and 1,427 (before 3,260).
+//    15.5 TFLOP/s (128 x 1,024 x 4,608: 87 us, before 510).  Two tiles of either height fit an SM: a round of them costs 0.110 us
+//    (64 rows) or 0.205 us (128) per k, and a last round with at most one tile an SM 0.062 or 0.123: 500 x 3,072 x 1,024 115 us
+//    with 64 rows (before 178), 1,000 x 1,024 x 4,608 286 (before 546), 1,000 x 9,216 x 1,024 410 with 128 rows (before 897),
+//    1,000 x 16,384 x 2,048 1,427 (before 3,260).
 static int launch_simt_float(float* Y, const float* X, const float* W, int M, int N, int K, long long ldx, long long ldw,
                              long long ldy, cudaStream_t st) {
     if (M <= 4 && N < 2048) return launch_simt_rows<4, 8>(Y, X, W, M, N, K, ldx, ldw, ldy, st);
@@ -411,11 +471,13 @@ static int launch_simt_float(float* Y, const float* X, const float* W, int M, in
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
         if (sm_count <= 0) sm_count = 1;
     }
-    const double cols = (N + GST_BN - 1) / GST_BN;
-    const double per_sm64 = cols * ((M + 63) / 64) / sm_count, per_sm128 = cols * ((M + 127) / 128) / sm_count;
+    const long long cols = (N + GST_BN - 1) / GST_BN, round = 2LL * sm_count;
+    auto tiles_us = [&](long long tiles, double full, double half) {
+        const long long left = tiles % round;
+        return K * (tiles / round * full + (left == 0 ? 0.0 : left <= sm_count ? half : full));
+    };
     const double rows = 2.0 * ((M + 7) / 8 * 8) * N * K / 15.5e6;
-    const double tile64 = K * (per_sm64 > 0.087 / 0.056 ? 0.056 * per_sm64 : 0.087);
-    const double tile128 = K * (per_sm128 > 0.123 / 0.1 ? 0.1 * per_sm128 : 0.123);
+    const double tile64 = tiles_us(cols * ((M + 63) / 64), 0.110, 0.062), tile128 = tiles_us(cols * ((M + 127) / 128), 0.205, 0.123);
     // (a grid has at most 65,535 rows of blocks, which ends the passes of eight at half a million rows)
     if (rows <= tile64 && rows <= tile128 && M <= 8 * 65535) return launch_simt_rows<8, 16>(Y, X, W, M, N, K, ldx, ldw, ldy, st);
     if (tile64 <= tile128 && M <= 64 * 65535) return launch_simt_tile<64>(Y, X, W, M, N, K, ldx, ldw, ldy, st);
