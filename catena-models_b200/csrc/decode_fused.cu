@@ -23,7 +23,7 @@
 //
 // Measured on B200 (LFM3 1.7B-class, decode at batch 8, 2,048 tokens of context): 37 launches a step
 // instead of 173, but 1.53 ms a step against 1.13 ms for the chain of single kernels replayed from a
-// graph.  A barrier phase costs as much as a kernel boundary (3.2 us for the residual + norm
+// graph (0.99 ms since their products stream through rings of their own).  A barrier phase costs as much as a kernel boundary (3.2 us for the residual + norm
 // operation, of which 0.8 us the fence and the arrival and 0.5 us the wait), and the ring does not
 // hide it: a group's loop over 4 KB stages (two barriers of its four warps, two shared-memory
 // reads, two mma) sustains about 11 KB/us, so a product whose items keep 65 % of the groups busy
